@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) attn_shared_tc_kernel(const TcA
 #pragma unroll
       for (int i = 0; i < 64; ++i) cur[i] = nxt[i];
     }
-  } else if (lane == 0) {
+  } else if (pi_elect()) {
     // ---- MMA issuer ------------------------------------------------------------------------------------------------
     auto idesc = [](uint32_t n) { return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((uint32_t)(kRowsTc >> 4) << 24); };
     const uint32_t id64 = idesc(64);

@@ -450,6 +450,16 @@ struct pi_smem_grant {
 };
 
 #ifdef __CUDACC__
+// True in one thread of a converged warp.  Single-thread work of the tensor pipe and the copy engine hangs off this instruction and
+// not off a lane number: only behind it the compiler knows that one thread is active and keeps descriptors in uniform
+// registers; behind `lane == 0` it issues every tcgen05.mma through a loop over the active threads (M 128, A in tensor memory,
+// whatever N: 130 cycles an instruction, against 35 at N 64, 72 at N 128, 104 at N 192).
+__device__ __forceinline__ bool pi_elect() {
+  uint32_t one;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+  return one != 0;
+}
+
 // y = p0 + p1 + p2 exactly, each a bf16 (each remainder has at most 16, then 8 significant bits left).
 __device__ __forceinline__ void pi_split3(float y, unsigned short& p0, unsigned short& p1, unsigned short& p2) {
   const __nv_bfloat16 a = __float2bfloat16_rn(y);

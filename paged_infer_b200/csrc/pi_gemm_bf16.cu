@@ -248,7 +248,7 @@ gemm_bf16_kernel(const Bf16GemmParams p, const __grid_constant__ CUtensorMap map
 
   if (warp == kEpiWarps) {
     // ---- TMA ------------------------------------------------------------------------------------------------------
-    if (lane == 0) {
+    if (pi_elect()) {
       if (GROUPED) {
         pi_grid_dependency_wait();
         s_dep_ok = 1;
@@ -283,7 +283,7 @@ gemm_bf16_kernel(const Bf16GemmParams p, const __grid_constant__ CUtensorMap map
     }
   } else if (warp == kEpiWarps + 1) {
     // ---- MMA ------------------------------------------------------------------------------------------------------
-    if (lane == 0) {
+    if (pi_elect()) {
       if (GROUPED) {
         pi_grid_dependency_wait();
         my_tiles = count(*p.n_tiles * p.rtiles);

@@ -168,7 +168,7 @@ gemm_ta_kernel(const GemmParams p, const __grid_constant__ CUtensorMap map_act) 
     asm volatile("bar.sync 1, %0;" ::"n"(kProducerWarps * 32) : "memory");
   } else if (warp == kProducerWarps) {
     // ---- activation loader: one 3-D TMA box {64 K, BN rows, 3 planes} per K atom -------------------------------
-    if (lane == 0) {
+    if (pi_elect()) {
       pi_grid_dependency_wait();  // the activation planes come from the preceding kernel
       s_dep_ok = 1;
       for (int kb = kb_begin; kb < kb_end; ++kb) {
@@ -194,7 +194,7 @@ gemm_ta_kernel(const GemmParams p, const __grid_constant__ CUtensorMap map_act) 
     }
   } else {
     // ---- MMA issuer ------------------------------------------------------------------------------------------
-    if (lane == 0) {
+    if (pi_elect()) {
       // kind::f16, D = f32, A (TMEM) and B (shared, K-major) = bf16, N = 3*BN, M = 128
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kDCols >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
       bool ok = true;
