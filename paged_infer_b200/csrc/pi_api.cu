@@ -173,7 +173,7 @@ void pi_ctx_destroy(pi_ctx* ctx) {
   cudaSetDevice(ctx->device);
   cudaStreamSynchronize(ctx->stream);
   pi_tp_destroy(ctx);
-  for (pi_buffer* b : {&ctx->staging_in, &ctx->staging_out, &ctx->attn_tables, &ctx->attn_partial, &ctx->attn_plan, &ctx->gemm_act})
+  for (pi_buffer* b : {&ctx->staging_in, &ctx->staging_out, &ctx->attn_tables, &ctx->attn_partial, &ctx->attn_plan, &ctx->gemm_act, &ctx->gemm_parked})
     if (b->ptr) cudaFree(b->ptr);
   if (ctx->pinned) cudaFreeHost(ctx->pinned);
   for (cudaEvent_t e : ctx->prof_events) cudaEventDestroy(e);
@@ -444,7 +444,7 @@ pi_status pi_linear_read_i8(pi_ctx* ctx, const pi_linear* lin, int8_t* q_host_ou
 }  // extern "C"
 
 pi_status pi_linear_forward(pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a) {
-  if (ctx->opt_tensor_gemm && a.M > ctx->opt_gemv_max_m && pi_gemm_tc_supported(ctx, lin, a)) return pi_launch_gemm_tc(ctx, lin, a);
+  if (pi_gemm_tc_will_run(ctx, lin, a) && pi_gemm_tc_scratch_ready(ctx, lin, a)) return pi_launch_gemm_tc(ctx, lin, a);
   return pi_launch_gemv(ctx, lin, a);
 }
 

@@ -117,6 +117,7 @@ struct pi_ctx {
   pi_buffer attn_partial;              // split-KV partial (m, l, acc)
   pi_buffer attn_plan;                 // flat work list of the step: segment ranges, segments, merge info, counters
   pi_buffer gemm_act;                  // bf16 activation planes (+ row factors) for the tensor GEMM
+  pi_buffer gemm_parked;               // wide tensor GEMM: ticket counters (zero between launches) and the parts of cut tiles
   std::vector<uint8_t> scratch_block_marks;   // host: physical blocks written by the step being staged
   void* pinned = nullptr;              // pinned host staging
   size_t pinned_bytes = 0;
@@ -297,9 +298,12 @@ struct pi_linear_args {
 pi_status pi_launch_gemm_bf16(pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a);
 // CUDA-core dequant GEMV/GEMM (any shape, any M).
 pi_status pi_launch_gemv(pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a);
-// tcgen05 tensor-core GEMM for int8 weights (returns PI_ERR_UNSUPPORTED when the shape does not fit).
+// tcgen05 tensor-core GEMM for int8 and bf16 weights (returns PI_ERR_UNSUPPORTED when the shape does not fit).
 pi_status pi_launch_gemm_tc(pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a);
 bool pi_gemm_tc_supported(const pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a);
+// False where a call with bf16 weights would have to allocate while its stream is captured: the CUDA-core kernel, which needs no
+// scratch, takes it.
+bool pi_gemm_tc_scratch_ready(const pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a);
 // True when pi_linear_forward would take the tensor-core path for this call.
 bool pi_gemm_tc_will_run(const pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a);
 // True when that launch can also emit planes (and, with a norm weight, the partial sums of squares).
@@ -460,10 +464,15 @@ __device__ __forceinline__ bool pi_elect() {
   return one != 0;
 }
 
-// y = p0 + p1 + p2 exactly, each a bf16 (each remainder has at most 16, then 8 significant bits left).
+// y = p0 + p1 + p2 exactly, each a bf16 (each remainder has at most 16, then 8 significant bits left).  p0 is rounded towards
+// zero where rounding to nearest would overflow; infinities and NaN are all in p0, so that they reach the sum as they are.
 __device__ __forceinline__ void pi_split3(float y, unsigned short& p0, unsigned short& p1, unsigned short& p2) {
-  const __nv_bfloat16 a = __float2bfloat16_rn(y);
-  const float r1 = y - __bfloat162float(a);
+  __nv_bfloat16 a = __float2bfloat16_rn(y);
+  float r1 = y - __bfloat162float(a);
+  if ((__float_as_uint(y) & 0x7fffffffu) >= 0x7f7f8000u) {
+    if (isfinite(y)) a = __float2bfloat16_rz(y);
+    r1 = isfinite(y) ? y - __bfloat162float(a) : 0.f;
+  }
   const __nv_bfloat16 b = __float2bfloat16_rn(r1);
   const float r2 = r1 - __bfloat162float(b);
   const __nv_bfloat16 c = __float2bfloat16_rn(r2);

@@ -70,7 +70,7 @@ gemm_ta_kernel(const GemmParams p, const __grid_constant__ CUtensorMap map_act) 
   __shared__ uint32_t s_tmem;
   __shared__ volatile int s_abort;
   __shared__ volatile int s_dep_ok;   // the preceding kernel has completed: from here on waits are this kernel's own
-  __shared__ float s_rowf[BN];     // row factor of the activation rows of this CTA
+  __shared__ EpiPlace s_place[BN];   // row factors of this CTA's activation rows and their places
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int quad = warp & 3, kq = (warp >> 2) & 3, half = (warp >> 2) & 1;
@@ -164,7 +164,7 @@ gemm_ta_kernel(const GemmParams p, const __grid_constant__ CUtensorMap map_act) 
     }
     pi_grid_dependency_wait();  // the epilogue below touches memory the producer kernel may still be writing
     // row factors of this CTA's activation rows (1/rms from the partial sums of squares, in tile order)
-    if (tid < BN) s_rowf[tid] = act_row_factor(p, m0 + tid);
+    if (tid < BN) epi_place(p, m0 + tid, s_place[tid]);
     asm volatile("bar.sync 1, %0;" ::"n"(kProducerWarps * 32) : "memory");
   } else if (warp == kProducerWarps) {
     // ---- activation loader: one 3-D TMA box {64 K, BN rows, 3 planes} per K atom -------------------------------
@@ -308,7 +308,7 @@ gemm_ta_kernel(const GemmParams p, const __grid_constant__ CUtensorMap map_act) 
         } else {
           acc = *reinterpret_cast<const float4*>(my_part + c * kBM + r4);
         }
-        epi_row(p, rows, blockIdx.x, m0 + c, s_rowf[c], acc, tid & 31);
+        epi_row(p, rows, blockIdx.x, m0 + c, s_place[c], acc, epi_old(p, rows, m0 + c), tid & 31);
       }
     }
     // nobody reads or writes a peer's shared memory after the barrier above: a CTA may leave as soon as it is done
@@ -536,7 +536,7 @@ pi_status build_gemm_params(pi_ctx* ctx, const pi_linear* lin, const pi_linear_a
                             GemmParams* out, CUtensorMap* map) {
   const int M = a.M, K = (int)lin->cols, N = (int)lin->rows;
   const int rtiles = (N + kBM - 1) / kBM;
-  const int nkb = K / kBK;
+  const int nkb = K / kBK;   // of pi_gemm_tc.cu's K blocks
   PI_REQUIRE(ctx, in.K == K && in.base, "activation planes do not match the projection (%d columns, planes of %d)", K, in.K);
 
   // one map over the three planes: {K, M rows (rows past M read as zero), 3 planes plane_stride apart}
@@ -553,8 +553,8 @@ pi_status build_gemm_params(pi_ctx* ctx, const pi_linear* lin, const pi_linear_a
 
   GemmParams pp = {};
   GemmParams& p = pp;
-  p.W = static_cast<const int8_t*>(lin->w);
-  p.scales = lin->scales;
+  p.W = lin->w;
+  p.scales = lin->kind == PI_INT8 ? lin->scales : nullptr;
   p.out = a.out;
   p.ld = lin->ld;
   p.out_stride = a.out_stride;
@@ -629,6 +629,7 @@ namespace {
 // The GEMM proper over activations that already are planes.
 pi_status run_gemm(pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a, const pi_act_planes& in) {
   const int M = a.M, K = (int)lin->cols, N = (int)lin->rows;
+  if (lin->kind == PI_BF16) return run_gemm_wide(ctx, lin, a, in);
   const int BN = pick_bn(M);
   const int mtiles = (M + BN - 1) / BN;
   const int rtiles = (N + kBM - 1) / kBM;
@@ -659,6 +660,8 @@ pi_status run_gemm(pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a, c
   return PI_OK;
 }
 
+size_t act_scratch_bytes(int M, int K) { return (size_t)kPlanes * M * K * sizeof(__nv_bfloat16) + (size_t)M * sizeof(float) + 256; }
+
 // Scratch layout shared by pi_launch_gemm_tc and pi_linear_apply_noalloc: [3 planes of rows x K bf16 | rows factors].
 pi_act_planes planes_in_scratch(void* scratch, int rows, int K) {
   pi_act_planes pl;
@@ -673,13 +676,33 @@ pi_act_planes planes_in_scratch(void* scratch, int rows, int K) {
 
 bool pi_gemm_tc_supported(const pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a) {
   (void)ctx;
-  if (lin->kind != PI_INT8) return false;
-  if (lin->cols % kBK != 0 || lin->ld != lin->cols) return false;   // whole K blocks, 32-byte aligned rows
-  if ((uintptr_t)lin->w % 32 != 0) return false;
+  if (a.epi != PI_EPI_STORE && a.epi != PI_EPI_ADD && a.epi != PI_EPI_SWIGLU) return false;
+  if (lin->kind == PI_INT8) {
+    if (lin->cols % kBK != 0 || lin->ld != lin->cols) return false;   // whole K blocks, 32-byte aligned rows
+    if ((uintptr_t)lin->w % 32 != 0) return false;
+  } else if (lin->kind == PI_BF16) {
+    if (lin->cols % 8 != 0 || lin->ld != lin->cols || (uintptr_t)lin->w % 16 != 0) return false;   // rows on 16-byte boundaries
+    // The CUDA-core kernel takes about 4 us and 0.37 us per million weights and pass over four rows, the split and the
+    // tensor-core GEMM 13 us and 0.5 us per million weights, whatever the batch: the lines cross where a million weights
+    // times (3 passes - 4) reach 70.  Both sides, us: 2048 x 2048, 32 rows (84) 17.9 and 16.2, 16 rows (34) 10.6 and 14.7;
+    // 11264 x 2048, 8 rows (46) 21.7 and 23.9, 16 rows (185) 39.9 and 24.6; 24000 x 5600, 5 rows (269) 104 and 77.
+    const double weights = (double)lin->rows * (double)lin->cols, passes = (a.M + 3) / 4;
+    if (weights * (3 * passes - 4) < 70e6) return false;
+    if (weights * ((a.M + 63) / 64) >= 8e12) return false;   // K blocks of a launch are counted in 32 bits
+  } else {
+    return false;
+  }
   if (lin->rows < 32) return false;
   if (a.epi == PI_EPI_SWIGLU && (lin->rows % 2) != 0) return false;
   if (lin->cols > 65536 * 2) return false;
   return encode_tiled() != nullptr;
+}
+
+bool pi_gemm_tc_scratch_ready(const pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a) {
+  if (lin->kind != PI_BF16 || a.in_planes) return true;
+  if (ctx->gemm_parked.ptr && ctx->gemm_act.bytes >= act_scratch_bytes(a.M, (int)lin->cols)) return true;
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(ctx->stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
 }
 
 bool pi_gemm_tc_will_run(const pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a) {
@@ -744,7 +767,7 @@ pi_status pi_launch_gemm_tc(pi_ctx* ctx, const pi_linear* lin, const pi_linear_a
   }
   const int M = a.M, K = (int)lin->cols;
   // scratch (global memory beyond the inputs and outputs): the planes and the row factors
-  PI_TRY(pi_reserve(ctx, &ctx->gemm_act, (size_t)kPlanes * M * K * sizeof(__nv_bfloat16) + (size_t)M * sizeof(float) + 256));
+  PI_TRY(pi_reserve(ctx, &ctx->gemm_act, act_scratch_bytes(M, K)));
   pi_act_planes pl = planes_in_scratch(ctx->gemm_act.ptr, M, K);
   {
     pi_prof_scope prof(ctx, PI_PROF_OTHER);
@@ -816,7 +839,7 @@ extern "C" pi_status pi_linear_apply_noalloc(pi_ctx* ctx, const pi_linear* lin, 
   a.out = out_dev;
   a.out_stride = lin->rows;
   a.M = M;
-  PI_REQUIRE(ctx, pi_gemm_tc_supported(ctx, lin, a),
+  PI_REQUIRE(ctx, lin->kind == PI_INT8 && pi_gemm_tc_supported(ctx, lin, a),
              "the allocation-free projection needs an int8 matrix with at least 32 rows and a multiple of 128 columns");
   void* scratch = nullptr;
   PI_TRY(noalloc_scratch_address(ctx, &scratch));

@@ -22,8 +22,8 @@ constexpr int kACols = kBK / 2;     // 128 bf16 of a weight row = 64 32-bit TMEM
 constexpr size_t kMinSmem = 120 * 1024;
 
 struct GemmParams {
-  const int8_t* W;
-  const float* scales;      // [N]
+  const void* W;            // int8, or bf16 (pi_gemm_wide.cu)
+  const float* scales;      // [N], null: 1 (bf16 weights)
   float* out;
   size_t ld, out_stride;
   int N, K, M;
@@ -69,6 +69,16 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+// One look at a phase, without waiting.  The answer takes about 190 cycles, also when it is yes: ask before other work.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return done != 0;
+}
 // Bounded wait; false when the limit ran out.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   for (uint32_t spin = 0; spin < kSpinLimit; ++spin) {
@@ -107,18 +117,16 @@ __device__ __forceinline__ void ld_stream_32(const void* p, uint32_t* v) {
                : "l"(p));
 }
 
-// 4 int8 -> 4 bf16 (exact): byte b^0x80 into the mantissa of 2^23 as f32, minus (2^23 + 128); an integer of at
-// most 8 significant bits has a zero low half as f32, so its upper 16 bits are the bf16 value.
+// 4 int8 -> 4 bf16 (exact).  With the sign bit s and the low seven bits m of a code, 0x4300 | m is 128 + m and
+// 0x4300 | s << 7 is 128 + 128 s; their difference m - 128 s is the code.  Two byte permutations per four codes, where
+// the way through the mantissa of 2^23 takes six.
 __device__ __forceinline__ void widen4(uint32_t w, uint32_t& lo, uint32_t& hi) {
-  const uint32_t x = w ^ 0x80808080u;
-  const float2 f01 = make_float2(__uint_as_float(__byte_perm(x, 0x4B000000u, 0x7650)),
-                                 __uint_as_float(__byte_perm(x, 0x4B000000u, 0x7651)));
-  const float2 f23 = make_float2(__uint_as_float(__byte_perm(x, 0x4B000000u, 0x7652)),
-                                 __uint_as_float(__byte_perm(x, 0x4B000000u, 0x7653)));
-  const float2 bias = make_float2(-8388736.0f, -8388736.0f);
-  const float2 a = __fadd2_rn(f01, bias), b = __fadd2_rn(f23, bias);
-  lo = __byte_perm(__float_as_uint(a.x), __float_as_uint(a.y), 0x7632);
-  hi = __byte_perm(__float_as_uint(b.x), __float_as_uint(b.y), 0x7632);
+  const uint32_t t0 = __byte_perm(w, 0x43u, 0x4140), t1 = __byte_perm(w, 0x43u, 0x4342);
+  const uint32_t m0 = t0 & 0xff7fff7fu, s0 = t0 & 0xff80ff80u, m1 = t1 & 0xff7fff7fu, s1 = t1 & 0xff80ff80u;
+  const __nv_bfloat162 a = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&m0), *reinterpret_cast<const __nv_bfloat162*>(&s0));
+  const __nv_bfloat162 b = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&m1), *reinterpret_cast<const __nv_bfloat162*>(&s1));
+  lo = *reinterpret_cast<const uint32_t*>(&a);
+  hi = *reinterpret_cast<const uint32_t*>(&b);
 }
 
 // Shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row groups 1024 bytes apart.
@@ -176,18 +184,46 @@ __device__ __forceinline__ float silu_mul(float g, float u) { return (g / (1.0f 
 
 __device__ __forceinline__ void split3(float y, unsigned short& p0, unsigned short& p1, unsigned short& p2) { pi_split3(y, p0, p1, p2); }
 
+// Row factor of activation row m: given, or 1/rms from the per-tile partial sums of squares (added in tile order), or 1.
+__device__ __forceinline__ float act_row_factor(const GemmParams& p, int m) {
+  float f = 1.0f;
+  if (m < p.M) {
+    if (p.act_scale) {
+      f = __ldcg(p.act_scale + m);
+    } else if (p.sumsq_in) {
+      float t = 0.f;
+      for (int i = 0; i < p.sumsq_tiles; ++i) t += __ldcg(p.sumsq_in + (size_t)i * p.sumsq_stride + m);
+      f = 1.0f / sqrtf(t / (float)p.K + p.eps);
+    }
+  }
+  return f;
+}
+
+// What the epilogue needs to know of an activation row: its factor, and where the rotary path finds and puts it.
+struct EpiPlace {
+  float factor;
+  int pos, block, off;   // block -1: unmapped
+};
+__device__ __forceinline__ void epi_place(const GemmParams& p, int m, EpiPlace& e) {
+  e.factor = act_row_factor(p, m);
+  if (!p.rope_hd) return;
+  e.pos = m < p.M ? p.pos[m] : 0;
+  const int lb = e.pos / p.L.block_size;
+  e.off = e.pos % p.L.block_size;
+  e.block = m < p.M && lb < p.lens[m] ? p.tables[(size_t)m * p.max_blocks + lb] : -1;
+}
+
 // Epilogue of the fused [q;k;v] projection: thread = four adjacent output columns rr..rr+3 of activation row m,
 // all 32 lanes of the warp on the same m (so the shuffles below are safe).  Row tiles are whole heads: the NeoX
 // partner (j, j + hd/2) of a lane's four values sits in lane ^ (hd/8), interleaved pairs (2j, 2j+1) are the
 // thread's own.  q: rotated into out.  k: rotated into out and into the pool.  v: copied into the pool.
-__device__ __forceinline__ void emit_rope(const GemmParams& p, int m, int rr, int lane, float v0, float v1, float v2, float v3) {
+__device__ __forceinline__ void emit_rope(const GemmParams& p, int m, const EpiPlace& at, int rr, int lane, float v0, float v1, float v2, float v3) {
   const int hd = p.rope_hd, half = hd >> 1;
   const bool valid = m < p.M && rr < p.N;
-  const int mm = valid ? m : 0;
   const int seg = rr < p.rope_q_rows ? 0 : (rr < p.rope_q_rows + p.rope_kv_rows ? 1 : 2);   // q, k, v
   const int within = rr - (seg == 0 ? 0 : (seg == 1 ? p.rope_q_rows : p.rope_q_rows + p.rope_kv_rows));
   const int d = within % hd;             // first of this thread's four dims inside its head
-  const int position = p.pos[mm];
+  const int position = at.pos;
   float r[4] = {v0, v1, v2, v3};
   if (p.rope_style == 0) {
     const int plane = hd >> 3;            // partner lane distance
@@ -213,11 +249,9 @@ __device__ __forceinline__ void emit_rope(const GemmParams& p, int m, int rr, in
   if (!valid) return;
   *reinterpret_cast<float4*>(p.out + (size_t)m * p.out_stride + rr) = make_float4(r[0], r[1], r[2], r[3]);
   if (seg == 0) return;
-  const int lb = position / p.L.block_size, off = position % p.L.block_size;
-  if (lb >= p.lens[m]) return;             // unmapped: the write is skipped silently
-  const int pb = p.tables[(size_t)m * p.max_blocks + lb];
+  if (at.block < 0) return;                // unmapped: the write is skipped silently
   const int kh = within / hd;
-  float* dst = p.kv + pi_kv_tile_offset(p.L, p.layer, pb, kh, seg == 2 ? 1 : 0) + (size_t)off * hd + d;
+  float* dst = p.kv + pi_kv_tile_offset(p.L, p.layer, at.block, kh, seg == 2 ? 1 : 0) + (size_t)at.off * hd + d;
   *reinterpret_cast<float4*>(dst) = make_float4(r[0], r[1], r[2], r[3]);
 }
 
@@ -235,7 +269,7 @@ __device__ __forceinline__ void epi_rows_load(const GemmParams& p, int row0, int
   e.rr = row0 + (tid & 31) * 4;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    e.wsc[i] = (e.rr + i < p.N) ? __ldg(p.scales + e.rr + i) : 0.f;
+    e.wsc[i] = (e.rr + i < p.N) ? (p.scales ? __ldg(p.scales + e.rr + i) : 1.0f) : 0.f;
     e.nw[i] = 1.0f;
   }
   if (p.emit_base && p.emit_norm) {
@@ -251,14 +285,23 @@ __device__ __forceinline__ void epi_rows_load(const GemmParams& p, int row0, int
   }
 }
 
-// One activation row m of the thread's four columns: acc = the raw dot products (all K, all planes added), `as` the
-// row factor of the activations.  All 32 lanes of a warp call this with the same m (the rotary path and the sum of
+// The residual that PI_EPI_ADD adds to the thread's four columns of row m, when the row's pieces are whole 16-byte groups
+// (epi_row reads it by itself where they are not).
+__device__ __forceinline__ float4 epi_old(const GemmParams& p, const EpiRows& e, int m) {
+  if (p.epi != PI_EPI_ADD || m >= p.M || e.rr + 3 >= p.N || (p.out_stride & 3) != 0 || (reinterpret_cast<uintptr_t>(p.out) & 15) != 0)
+    return make_float4(0.f, 0.f, 0.f, 0.f);
+  return __ldcg(reinterpret_cast<const float4*>(p.out + (size_t)m * p.out_stride + e.rr));
+}
+
+// One activation row m of the thread's four columns: acc = the raw dot products (all K, all planes added), `at` the
+// row's place, `old` from epi_old.  All 32 lanes of a warp call this with the same m (the rotary path and the sum of
 // squares shuffle across the warp).  `tile` is the row tile (index of the per-tile sums of squares).  The residual
 // is read past L1: inside a persistent kernel another SM may have written it a moment ago.
-__device__ __forceinline__ void epi_row(const GemmParams& p, const EpiRows& e, int tile, int m, float as, float4 acc, int lane) {
+__device__ __forceinline__ void epi_row(const GemmParams& p, const EpiRows& e, int tile, int m, const EpiPlace& at, float4 acc, float4 old, int lane) {
   const int rr = e.rr;
+  const float as = at.factor;
   if (p.rope_hd) {   // fused [q;k;v] projection: rotary embedding + KV write
-    emit_rope(p, m, rr, lane, acc.x * e.wsc[0] * as, acc.y * e.wsc[1] * as, acc.z * e.wsc[2] * as, acc.w * e.wsc[3] * as);
+    emit_rope(p, m, at, rr, lane, acc.x * e.wsc[0] * as, acc.y * e.wsc[1] * as, acc.z * e.wsc[2] * as, acc.w * e.wsc[3] * as);
     return;
   }
   float sq = 0.f;
@@ -288,7 +331,6 @@ __device__ __forceinline__ void epi_row(const GemmParams& p, const EpiRows& e, i
       const bool full = rr + 3 < p.N;
       if (full && ((p.out_stride & 3) == 0) && ((reinterpret_cast<uintptr_t>(p.out) & 15) == 0)) {
         if (add) {
-          const float4 old = __ldcg(reinterpret_cast<const float4*>(o));
           r[0] += old.x; r[1] += old.y; r[2] += old.z; r[3] += old.w;
         }
         *reinterpret_cast<float4*>(o) = make_float4(r[0], r[1], r[2], r[3]);
@@ -322,22 +364,6 @@ __device__ __forceinline__ void epi_row(const GemmParams& p, const EpiRows& e, i
   }
 }
 
-// Row factor of activation row m: given, or 1/rms from the per-tile partial sums of squares (added in tile order), or 1.
-__device__ __forceinline__ float act_row_factor(const GemmParams& p, int m) {
-  float f = 1.0f;
-  if (m < p.M) {
-    if (p.act_scale) {
-      f = __ldcg(p.act_scale + m);
-    } else if (p.sumsq_in) {
-      float t = 0.f;
-      for (int i = 0; i < p.sumsq_tiles; ++i) t += __ldcg(p.sumsq_in + (size_t)i * p.sumsq_stride + m);
-      f = 1.0f / sqrtf(t / (float)p.K + p.eps);
-    }
-  }
-  return f;
-}
-
-
 // ---- host side (pi_gemm_tc.cu) ----------------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -350,5 +376,7 @@ int pick_bn(int M);
 // ({K, M rows, 3 planes}; rows past M read as zero).  Also fills in what `a.emit` hands to the next projection.
 pi_status build_gemm_params(pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a, const pi_act_planes& in, int BN,
                             GemmParams* p, CUtensorMap* map);
+// The projection over planes for bf16 weights (pi_gemm_wide.cu).
+pi_status run_gemm_wide(pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a, const pi_act_planes& in);
 
 }  // namespace pi_tc
