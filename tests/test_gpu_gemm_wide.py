@@ -28,7 +28,7 @@ def bf16_matrix(rows, cols, seed):
 
 # one tile; a row more; K that ends inside a block and off the 32-byte grid; fewer tiles than SMs, each shared; more
 @pytest.mark.parametrize("rows,cols,M", [(128, 4096, 512), (129, 5608, 449), (2048, 1000, 129), (2047, 2056, 64), (2560, 2048, 65), (11264, 2048, 9),
-                                         (24000, 1400, 5), (32000, 2048, 130), (40, 65536, 300)])
+                                         (24000, 1608, 5), (32000, 2048, 130), (40, 65536, 300)])
 def test_bf16_weights(ctx, rows, cols, M):
     from paged_infer_b200 import api
     bits, w = bf16_matrix(rows, cols, rows + M)
