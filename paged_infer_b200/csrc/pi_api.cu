@@ -444,7 +444,7 @@ pi_status pi_linear_read_i8(pi_ctx* ctx, const pi_linear* lin, int8_t* q_host_ou
 }  // extern "C"
 
 pi_status pi_linear_forward(pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a) {
-  if (pi_gemm_tc_will_run(ctx, lin, a) && pi_gemm_tc_scratch_ready(ctx, lin, a)) return pi_launch_gemm_tc(ctx, lin, a);
+  if (pi_gemm_tc_will_run(ctx, lin, a)) return pi_launch_gemm_tc(ctx, lin, a);
   return pi_launch_gemv(ctx, lin, a);
 }
 
@@ -460,6 +460,13 @@ pi_status pi_linear_apply(pi_ctx* ctx, const pi_linear* lin, const float* x_dev,
   a.out = out_dev;
   a.out_stride = lin->rows;
   a.M = M;
+  // A host's own graph outlives this call and may be replayed on any stream: with bf16 weights it holds the kernel that needs
+  // no scratch of the context, whatever ran before.
+  if (lin->kind == PI_BF16) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusActive;
+    if (cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess) cudaGetLastError();
+    if (st != cudaStreamCaptureStatusNone) return pi_launch_gemv(ctx, lin, a);
+  }
   return pi_linear_forward(ctx, lin, a);
 }
 

@@ -301,9 +301,6 @@ pi_status pi_launch_gemv(pi_ctx* ctx, const pi_linear* lin, const pi_linear_args
 // tcgen05 tensor-core GEMM for int8 and bf16 weights (returns PI_ERR_UNSUPPORTED when the shape does not fit).
 pi_status pi_launch_gemm_tc(pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a);
 bool pi_gemm_tc_supported(const pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a);
-// False where a call with bf16 weights would have to allocate while its stream is captured: the CUDA-core kernel, which needs no
-// scratch, takes it.
-bool pi_gemm_tc_scratch_ready(const pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a);
 // True when pi_linear_forward would take the tensor-core path for this call.
 bool pi_gemm_tc_will_run(const pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a);
 // True when that launch can also emit planes (and, with a norm weight, the partial sums of squares).

@@ -698,13 +698,6 @@ bool pi_gemm_tc_supported(const pi_ctx* ctx, const pi_linear* lin, const pi_line
   return encode_tiled() != nullptr;
 }
 
-bool pi_gemm_tc_scratch_ready(const pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a) {
-  if (lin->kind != PI_BF16 || a.in_planes) return true;
-  if (ctx->gemm_parked.ptr && ctx->gemm_act.bytes >= act_scratch_bytes(a.M, (int)lin->cols)) return true;
-  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(ctx->stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
-}
-
 bool pi_gemm_tc_will_run(const pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a) {
   return ctx->opt_tensor_gemm && a.M > ctx->opt_gemv_max_m && pi_gemm_tc_supported(ctx, lin, a);
 }

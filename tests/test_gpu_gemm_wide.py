@@ -61,3 +61,42 @@ def test_infinities_and_nan_stay_in_their_rows(ctx):
     assert np.array_equal(got[3], np.where(w[:, 7] > 0, np.inf, -np.inf).astype(np.float32))
     assert np.isnan(got[5]).all()
     np.testing.assert_allclose(got[8], w[:, 0] * x[8, 0], rtol=1e-6)
+
+
+@pytest.mark.parametrize("called_before", [False, True])
+def test_captured_projection_holds_no_scratch(called_before):
+    """A host's graph of a bf16 projection is the one kernel that keeps nothing in the context: the same bits whether or not the
+    context has run such calls before, and still after later calls of larger sizes."""
+    import torch
+
+    from paged_infer_b200 import api
+    M, rows, cols = 64, 2048, 2048                  # eager calls of this size run on the tensor pipe
+    bits, _ = bf16_matrix(rows, cols, 7)
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        ctx = api.Context(0, stream.cuda_stream)
+        p = api.Projection.f32(ctx, bits)
+        x = torch.zeros(M, cols, device="cuda")
+        out, want = torch.empty(M, rows, device="cuda"), torch.empty(M, rows, device="cuda")
+        ctx.set_option(1, 0)                        # PI_OPT_TENSOR_GEMM off: the CUDA-core kernel, and its set-up before the capture
+        p.apply_device(x, want, M)
+        ctx.set_option(1, 1)
+        if called_before:
+            p.apply_device(x, out, M)
+        ctx.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        before = ctx.kernel_launches()
+        with torch.cuda.graph(graph, stream=stream):
+            p.apply_device(x, out, M)
+        assert ctx.kernel_launches() - before == 1
+        larger = api.Projection.f32(ctx, bf16_matrix(2048, 4096, 8)[0])
+        for big in (256, 1024):
+            larger.apply_device(torch.ones(big, 4096, device="cuda"), torch.empty(big, 2048, device="cuda"), big)
+        x.copy_(torch.from_numpy(normal_f32((M, cols), 9, 1.0)))
+        graph.replay()
+        ctx.set_option(1, 0)
+        p.apply_device(x, want, M)
+        ctx.synchronize()
+        assert torch.equal(out, want)
+        del graph
+        ctx.close()
