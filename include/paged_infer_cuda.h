@@ -176,15 +176,23 @@ pi_status pi_linear_read_i8(pi_ctx* ctx, const pi_linear* lin, int8_t* q_host_ou
  * src/math.rs:473-512, and the f32 twin :93-129) and Projection::apply_batched
  * (src/model.rs:247-259; math::matmat_i8_weight_parallel, src/math.rs:223-275,
  * plus transpose_rb_to_br :281-290).  On a tensor-parallel context this applies
- * the local shard only (no all-reduce). */
+ * the local shard only (no all-reduce).
+ * Scratch: int8 matrices beyond a few rows use a buffer of the context that grows
+ * with cudaMalloc when a larger shape arrives (pi_linear_apply_noalloc does not).
+ * bf16 matrices have theirs from pi_linear_create_bf16 on (6 bytes x columns x 1024
+ * rows, 256 MiB at most, the largest of a context's matrices, and 10 MB once; where
+ * that much memory is not free the matrix is created all the same and stays on the
+ * CUDA cores); their calls allocate nothing and larger batches pass in portions.
+ * Captured into a CUDA graph, a bf16 projection runs on the CUDA cores and holds no
+ * scratch, so the graph stays valid as long as its matrix and buffers do. */
 pi_status pi_linear_apply(pi_ctx* ctx, const pi_linear* lin, const float* x_dev, float* out_dev, int M);
 /* Same with host buffers: copies x in, runs, copies out back, synchronises. */
 pi_status pi_linear_apply_host(pi_ctx* ctx, const pi_linear* lin, const float* x_host, float* out_host, int M);
 /* pi_linear_apply for callers that must not allocate while they run it.  This
  * entry point has no counterpart in the reference.  The tensor-core projection
  * keeps three bf16 planes of the activations and one factor per activation row
- * in scratch memory; pi_linear_apply grows that scratch with cudaMalloc when a
- * larger shape arrives.  A caller that is inside a CUDA stream capture, that has
+ * in scratch memory; for int8 matrices pi_linear_apply grows that scratch with
+ * cudaMalloc when a larger shape arrives.  A caller that is inside a CUDA stream capture, that has
  * a latency budget a driver allocation would break, or that has given all
  * device memory to its own pool cannot afford that, so this variant uses a
  * fixed scratch area built into the library (about 3 MiB, held by every GPU

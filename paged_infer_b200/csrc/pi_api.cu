@@ -1,5 +1,6 @@
 // C-ABI entry points: context, quantiser, projections, KV pool, attention and
 // the host-buffer glue calls.  The model forward lives in pi_model.cu.
+#include <limits.h>
 #include <stdarg.h>
 #include <string.h>
 
@@ -173,7 +174,8 @@ void pi_ctx_destroy(pi_ctx* ctx) {
   cudaSetDevice(ctx->device);
   cudaStreamSynchronize(ctx->stream);
   pi_tp_destroy(ctx);
-  for (pi_buffer* b : {&ctx->staging_in, &ctx->staging_out, &ctx->attn_tables, &ctx->attn_partial, &ctx->attn_plan, &ctx->gemm_act, &ctx->gemm_parked})
+  for (pi_buffer* b : {&ctx->staging_in, &ctx->staging_out, &ctx->attn_tables, &ctx->attn_partial, &ctx->attn_plan, &ctx->gemm_act, &ctx->wide_planes,
+                       &ctx->gemm_parked})
     if (b->ptr) cudaFree(b->ptr);
   if (ctx->pinned) cudaFreeHost(ctx->pinned);
   for (cudaEvent_t e : ctx->prof_events) cudaEventDestroy(e);
@@ -402,6 +404,8 @@ static pi_status create_plain(pi_ctx* ctx, int kind, size_t rows, size_t cols, c
   if (s != PI_OK) {
     pi_linear_destroy(*out);
     *out = nullptr;
+  } else {
+    pi_gemm_wide_reserve(ctx, *out, INT_MAX);
   }
   return s;
 }

@@ -116,7 +116,8 @@ struct pi_ctx {
   pi_buffer attn_tables;               // block tables + per-entry (len, pos, start)
   pi_buffer attn_partial;              // split-KV partial (m, l, acc)
   pi_buffer attn_plan;                 // flat work list of the step: segment ranges, segments, merge info, counters
-  pi_buffer gemm_act;                  // bf16 activation planes (+ row factors) for the tensor GEMM
+  pi_buffer gemm_act;                  // bf16 activation planes (+ row factors) for the tensor GEMM, int8 weights
+  pi_buffer wide_planes;               // the same for bf16 weights: sized when a matrix is created, no call touches its size
   pi_buffer gemm_parked;               // wide tensor GEMM: ticket counters (zero between launches) and the parts of cut tiles
   std::vector<uint8_t> scratch_block_marks;   // host: physical blocks written by the step being staged
   void* pinned = nullptr;              // pinned host staging
@@ -301,6 +302,9 @@ pi_status pi_launch_gemv(pi_ctx* ctx, const pi_linear* lin, const pi_linear_args
 // tcgen05 tensor-core GEMM for int8 and bf16 weights (returns PI_ERR_UNSUPPORTED when the shape does not fit).
 pi_status pi_launch_gemm_tc(pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a);
 bool pi_gemm_tc_supported(const pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a);
+// Scratch for tensor-core launches over this matrix of at most `rows` rows (bf16 weights; nothing for others).  Called where a
+// matrix is created, so that no call allocates; where memory is short the matrix stays on the CUDA-core kernel.
+void pi_gemm_wide_reserve(pi_ctx* ctx, const pi_linear* lin, int rows);
 // True when pi_linear_forward would take the tensor-core path for this call.
 bool pi_gemm_tc_will_run(const pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a);
 // True when that launch can also emit planes (and, with a norm weight, the partial sums of squares).

@@ -48,6 +48,7 @@
 namespace cg = cooperative_groups;
 
 #include "pi_gemm_tc.cuh"
+#include "pi_gemm_wide.cuh"
 
 namespace {
 using namespace pi_tc;
@@ -530,6 +531,10 @@ int pick_ksplit(pi_ctx* ctx, int BN, int tiles, int nkb) {
 
 namespace pi_tc {
 
+bool wide_fits(const pi_linear* lin) {   // rows on 16-byte boundaries
+  return lin->cols % 8 == 0 && lin->ld == lin->cols && (uintptr_t)lin->w % 16 == 0 && lin->rows >= kMinRows && lin->cols <= kMaxCols;
+}
+
 int pick_bn(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : 64; }
 
 pi_status build_gemm_params(pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a, const pi_act_planes& in, int BN,
@@ -660,7 +665,35 @@ pi_status run_gemm(pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a, c
   return PI_OK;
 }
 
-size_t act_scratch_bytes(int M, int K) { return (size_t)kPlanes * M * K * sizeof(__nv_bfloat16) + (size_t)M * sizeof(float) + 256; }
+// The rows first .. first + n of a call.
+struct row_range {
+  pi_linear_args a;
+  pi_act_planes emit;
+  pi_rope_kv rope;
+  pi_attn_batch batch;
+  row_range(const pi_linear_args& whole, int first, int n) : a(whole) {
+    a.M = n;
+    a.x += (size_t)first * a.x_stride;
+    a.out += (size_t)first * a.out_stride;
+    for (int i = 0; i < a.n_out_also; ++i) a.out_also[i] += (size_t)first * a.out_stride;
+    if (whole.emit) {
+      emit = *whole.emit;
+      emit.base += (size_t)first * emit.K;
+      if (emit.sumsq) emit.sumsq += first;
+      a.emit = &emit;
+    }
+    if (whole.rope) {
+      rope = *whole.rope;
+      batch = *rope.batch;
+      batch.tables += (size_t)first * batch.max_blocks;
+      batch.lens += first;
+      batch.pos += first;
+      rope.batch = &batch;
+      a.rope = &rope;
+    }
+  }
+  row_range(const row_range&) = delete;
+};
 
 // Scratch layout shared by pi_launch_gemm_tc and pi_linear_apply_noalloc: [3 planes of rows x K bf16 | rows factors].
 pi_act_planes planes_in_scratch(void* scratch, int rows, int K) {
@@ -675,13 +708,12 @@ pi_act_planes planes_in_scratch(void* scratch, int rows, int K) {
 }  // namespace
 
 bool pi_gemm_tc_supported(const pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a) {
-  (void)ctx;
   if (a.epi != PI_EPI_STORE && a.epi != PI_EPI_ADD && a.epi != PI_EPI_SWIGLU) return false;
   if (lin->kind == PI_INT8) {
     if (lin->cols % kBK != 0 || lin->ld != lin->cols) return false;   // whole K blocks, 32-byte aligned rows
     if ((uintptr_t)lin->w % 32 != 0) return false;
   } else if (lin->kind == PI_BF16) {
-    if (lin->cols % 8 != 0 || lin->ld != lin->cols || (uintptr_t)lin->w % 16 != 0) return false;   // rows on 16-byte boundaries
+    if (!wide_fits(lin)) return false;
     // The CUDA-core kernel takes about 4 us and 0.37 us per million weights and pass over four rows, the split and the
     // tensor-core GEMM 13 us and 0.5 us per million weights, whatever the batch: the lines cross where a million weights
     // times (3 passes - 4) reach 70.  Both sides, us: 2048 x 2048, 32 rows (84) 17.9 and 16.2, 16 rows (34) 10.6 and 14.7;
@@ -689,12 +721,12 @@ bool pi_gemm_tc_supported(const pi_ctx* ctx, const pi_linear* lin, const pi_line
     const double weights = (double)lin->rows * (double)lin->cols, passes = (a.M + 3) / 4;
     if (weights * (3 * passes - 4) < 70e6) return false;
     if (weights * ((a.M + 63) / 64) >= 8e12) return false;   // K blocks of a launch are counted in 32 bits
+    if (!ctx->gemm_parked.ptr || ctx->wide_planes.bytes < pi_wide::planes_bytes(pi_wide::portion_rows(a.M, lin->cols), lin->cols)) return false;
   } else {
     return false;
   }
-  if (lin->rows < 32) return false;
+  if (lin->rows < kMinRows || lin->cols > kMaxCols) return false;
   if (a.epi == PI_EPI_SWIGLU && (lin->rows % 2) != 0) return false;
-  if (lin->cols > 65536 * 2) return false;
   return encode_tiled() != nullptr;
 }
 
@@ -758,22 +790,33 @@ pi_status pi_launch_gemm_tc(pi_ctx* ctx, const pi_linear* lin, const pi_linear_a
     pi_prof_scope prof(ctx, PI_PROF_GEMM_TC);
     return run_gemm(ctx, lin, a, *a.in_planes);
   }
-  const int M = a.M, K = (int)lin->cols;
   // scratch (global memory beyond the inputs and outputs): the planes and the row factors
-  PI_TRY(pi_reserve(ctx, &ctx->gemm_act, act_scratch_bytes(M, K)));
-  pi_act_planes pl = planes_in_scratch(ctx->gemm_act.ptr, M, K);
-  {
-    pi_prof_scope prof(ctx, PI_PROF_OTHER);
-    PI_TRY(pi_launch_act_split(ctx, a.x, a.x_stride, a.norm_weight, a.norm_eps, M, K, &pl));
+  const int K = (int)lin->cols;
+  pi_buffer& scratch = lin->kind == PI_BF16 ? ctx->wide_planes : ctx->gemm_act;
+  if (lin->kind != PI_BF16) PI_TRY(pi_reserve(ctx, &scratch, pi_wide::planes_bytes(a.M, K)));
+  const int step = lin->kind == PI_BF16 ? pi_wide::portion_rows(a.M, K) : a.M;
+  for (int first = 0; first < a.M; first += step) {
+    row_range part(a, first, std::min(step, a.M - first));
+    pi_act_planes pl = planes_in_scratch(scratch.ptr, part.a.M, K);
+    {
+      pi_prof_scope prof(ctx, PI_PROF_OTHER);
+      PI_TRY(pi_launch_act_split(ctx, part.a.x, a.x_stride, a.norm_weight, a.norm_eps, part.a.M, K, &pl));
+    }
+    pi_prof_scope prof(ctx, PI_PROF_GEMM_TC);
+    PI_TRY(run_gemm(ctx, lin, part.a, pl));
+    if (a.emit) {   // what the launch says of its planes, for the whole
+      a.emit->row_scale = part.emit.row_scale;
+      a.emit->sumsq_tiles = part.emit.sumsq_tiles;
+      a.emit->eps = part.emit.eps;
+    }
   }
-  pi_prof_scope prof(ctx, PI_PROF_GEMM_TC);
-  return run_gemm(ctx, lin, a, pl);
+  return PI_OK;
 }
 
 // ---- pi_linear_apply_noalloc -----------------------------------------------------------------------------------
 //
 // The tensor-core projection needs scratch in global memory: the three bf16 planes the f32 activations are split
-// into, plus one factor per activation row.  pi_linear_apply takes that scratch from a buffer the context grows
+// into, plus one factor per activation row.  For int8 pi_linear_apply takes that scratch from a buffer the context grows
 // with cudaMalloc on demand.  Some callers must not allocate at the moment they run a projection: a serving loop
 // that is inside a CUDA stream capture (cudaMalloc is not a capturable operation and invalidates the capture), a
 // host thread with a latency budget that a driver allocation (which can take the device-wide allocation lock and

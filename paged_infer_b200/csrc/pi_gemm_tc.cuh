@@ -20,6 +20,7 @@ constexpr int kACols = kBK / 2;     // 128 bf16 of a weight row = 64 32-bit TMEM
 // Every CTA asks for all 512 TMEM columns and for at least this much shared memory, so two of these CTAs never share
 // an SM: a CTA blocked in tcgen05.alloc while its cluster peers wait for it at a cluster barrier could deadlock.
 constexpr size_t kMinSmem = 120 * 1024;
+constexpr size_t kMinRows = 32, kMaxCols = 131072;   // of the matrices that these kernels take
 
 struct GemmParams {
   const void* W;            // int8, or bf16 (pi_gemm_wide.cu)
@@ -376,6 +377,8 @@ int pick_bn(int M);
 // ({K, M rows, 3 planes}; rows past M read as zero).  Also fills in what `a.emit` hands to the next projection.
 pi_status build_gemm_params(pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a, const pi_act_planes& in, int BN,
                             GemmParams* p, CUtensorMap* map);
+// Whether the kernel for bf16 weights can read this matrix.
+bool wide_fits(const pi_linear* lin);
 // The projection over planes for bf16 weights (pi_gemm_wide.cu).
 pi_status run_gemm_wide(pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a, const pi_act_planes& in);
 

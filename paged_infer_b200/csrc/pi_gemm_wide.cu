@@ -271,6 +271,37 @@ gemm_wide_kernel(const GemmParams p, const Cut cut, float* __restrict__ parked, 
 
 }  // namespace
 
+void pi_gemm_wide_reserve(pi_ctx* ctx, const pi_linear* lin, int rows) {
+  if (lin->kind != PI_BF16 || !pi_tc::wide_fits(lin)) return;
+  // The tickets and the parts of cut tiles: of one size for every launch of the context; the tickets start and stay at zero
+  // between launches.
+  if (!ctx->gemm_parked.ptr) {
+    const size_t tickets = pi_wide::ticket_bytes(ctx->sm_count), bytes = tickets + (size_t)ctx->sm_count * 2 * kTileFloats * sizeof(float);
+    void* ptr = nullptr;
+    if (cudaMalloc(&ptr, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      return;
+    }
+    if (cudaMemsetAsync(ptr, 0, tickets, ctx->stream) != cudaSuccess) {
+      cudaGetLastError();
+      cudaFree(ptr);
+      return;
+    }
+    ctx->gemm_parked.ptr = ptr;
+    ctx->gemm_parked.bytes = bytes;
+  }
+  const size_t want = pi_wide::planes_bytes(std::min(rows, pi_wide::portion_limit(lin->cols)), lin->cols);
+  if (want <= ctx->wide_planes.bytes) return;
+  void* ptr = nullptr;
+  if (cudaStreamSynchronize(ctx->stream) != cudaSuccess || cudaMalloc(&ptr, want) != cudaSuccess) {   // what there is stays
+    cudaGetLastError();
+    return;
+  }
+  if (ctx->wide_planes.ptr) cudaFree(ctx->wide_planes.ptr);
+  ctx->wide_planes.ptr = ptr;
+  ctx->wide_planes.bytes = want;
+}
+
 pi_status pi_tc::run_gemm_wide(pi_ctx* ctx, const pi_linear* lin, const pi_linear_args& a, const pi_act_planes& in) {
   GemmParams p;
   CUtensorMap act, w;
@@ -284,11 +315,6 @@ pi_status pi_tc::run_gemm_wide(pi_ctx* ctx, const pi_linear* lin, const pi_linea
     if (r != CUDA_SUCCESS) return pi_fail(ctx, PI_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d", (int)r);
   }
   const Cut cut = pi_wide::make_cut((int)lin->rows, a.M, (int)lin->cols, ctx->sm_count);
-  if (!ctx->gemm_parked.ptr) {   // of one size for every launch of the context; the tickets start and stay at zero between launches
-    const size_t bytes = pi_wide::ticket_bytes(ctx->sm_count) + (size_t)ctx->sm_count * 2 * kTileFloats * sizeof(float);
-    PI_TRY(pi_reserve(ctx, &ctx->gemm_parked, bytes));
-    PI_CUDA(ctx, cudaMemsetAsync(ctx->gemm_parked.ptr, 0, pi_wide::ticket_bytes(ctx->sm_count), ctx->stream));
-  }
   static pi_smem_grant granted;
   if (kWideSmem > granted.of(ctx)) {
     PI_CUDA(ctx, cudaFuncSetAttribute(gemm_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWideSmem));

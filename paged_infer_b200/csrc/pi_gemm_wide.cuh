@@ -61,6 +61,25 @@ __host__ __device__ inline int holders(const Cut& c, int cta, int tile, int* slo
   return n;
 }
 
+// Scratch for the activations of a launch: three 16-bit planes and a factor per row.
+inline size_t planes_bytes(size_t rows, size_t cols) { return 3 * rows * cols * 2 + rows * sizeof(float) + 256; }
+
+// Activation rows that pass through the scratch at once, from the sizes of the call alone, so that a row's sums do not depend on
+// what a context has done before: all of them up to the limit, else equal portions of whole tiles.  The limit keeps the scratch
+// at 1024 rows and 256 MiB; 1024 rows are 16 tiles, beside whose products another reading of the matrix does not show.
+constexpr int kPortion = 1024;
+constexpr size_t kPlanesLimit = (size_t)256 << 20;
+inline int portion_limit(size_t cols) {
+  const size_t fit = (kPlanesLimit - 256) / (3 * cols * 2 + sizeof(float)) / kCols * kCols;
+  return (int)(fit < (size_t)kPortion ? fit : (size_t)kPortion);
+}
+inline int portion_rows(int M, size_t cols) {
+  const int limit = portion_limit(cols);
+  if (M <= limit) return M;
+  const int n = (M - 1) / limit + 1;
+  return ((M - 1) / n + kCols) / kCols * kCols;
+}
+
 __host__ __device__ inline size_t ticket_bytes(int sms) { return ((size_t)sms * sizeof(int) + 255) / 256 * 256; }
 
 }  // namespace pi_wide

@@ -296,6 +296,9 @@ pi_status build_model(pi_ctx* ctx, const pi_model_config* cfg, const ModelSource
     m->sumsq_tiles_cap = (hidden + 127) / 128;
     PI_TRY(alloc_f(ctx, &m->sumsq, (size_t)m->sumsq_tiles_cap * cap));
   }
+  for (int l = 0; l < NL; ++l)
+    for (const pi_linear* lin : {m->qkv[l], m->wo[l], m->gate_up[l], m->down[l]}) pi_gemm_wide_reserve(ctx, lin, m->capacity);
+  pi_gemm_wide_reserve(ctx, m->lm_head, m->capacity);
   PI_TRY(ensure_rope(ctx, m, cfg->max_positions > 0 ? cfg->max_positions : 4096));
   PI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return PI_OK;

@@ -100,3 +100,106 @@ def test_captured_projection_holds_no_scratch(called_before):
         assert torch.equal(out, want)
         del graph
         ctx.close()
+
+
+@pytest.mark.parametrize("rows,cols,M,portions", [(2048, 1024, 1024, 1), (2048, 1024, 2049, 3), (320, 65536, 700, 2)])
+def test_large_batches_pass_in_portions_and_allocate_nothing(rows, cols, M, portions):
+    """The planes of a batch have a bounded scratch, laid out when the matrix is created: no call of any size allocates, the first
+    one included, and a row's bits are those of the portion it is in."""
+    import torch
+
+    from paged_infer_b200 import api
+    bits, w = bf16_matrix(rows, cols, rows + M)
+    x = torch.from_numpy(normal_f32((M, cols), M, 1.0)).cuda()
+    out, part = torch.empty(M, rows, device="cuda"), torch.empty(M, rows, device="cuda")
+    want = x.double() @ torch.from_numpy(w).cuda().double().T
+    warm = api.Context(0)                               # what the driver sets aside for kernels that run for the first time
+    api.Projection.f32(warm, bits).apply_device(x, out, M)
+    warm.synchronize()
+    ctx = api.Context(0)
+    p = api.Projection.f32(ctx, bits)
+    torch.cuda.synchronize()
+    free, before = torch.cuda.mem_get_info()[0], ctx.kernel_launches()
+    p.apply_device(x, out, M)
+    ctx.synchronize()
+    assert torch.cuda.mem_get_info()[0] == free
+    assert ctx.kernel_launches() - before == 2 * portions
+    assert ((out - want).abs() / want.abs().maximum(want.square().mean(1, keepdim=True).sqrt())).max() < 2e-6
+    step = -(-(-(-M // portions)) // 64) * 64 if portions > 1 else M
+    for first in range(0, M, step):
+        n = min(step, M - first)
+        if n * 2 < step:                                # a short rest alone may lie on the other side of the dispatch line
+            continue
+        p.apply_device(x[first:first + n], part[first:first + n], n)
+        ctx.synchronize()
+        assert torch.equal(out[first:first + n], part[first:first + n])
+    ctx.close()
+    warm.close()
+
+
+def test_int8_graphs_survive_bf16_calls():
+    """bf16 projections leave the scratch that int8 ones use alone, also where a host's graph holds it."""
+    import torch
+
+    from paged_infer_b200 import api
+    M, rows, cols = 64, 2048, 1024
+    rng = np.random.default_rng(3)
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        ctx = api.Context(0, stream.cuda_stream)
+        p = api.Projection.int8(ctx, rng.integers(-127, 128, (rows, cols), dtype=np.int8), np.full(rows, 1e-3, np.float32))
+        x = torch.from_numpy(normal_f32((M, cols), 1, 1.0)).cuda()
+        out, want = torch.empty(M, rows, device="cuda"), torch.empty(M, rows, device="cuda")
+        p.apply_device(x, want, M)
+        ctx.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            p.apply_device(x, out, M)
+        wide = api.Projection.f32(ctx, bf16_matrix(2048, 4096, 8)[0])
+        wide.apply_device(torch.ones(256, 4096, device="cuda"), torch.empty(256, 2048, device="cuda"), 256)
+        graph.replay()
+        ctx.synchronize()
+        assert torch.equal(out, want)
+        del graph
+        ctx.close()
+
+
+def bf16_llama(ctx, seed, hidden, heads, kv_heads, inter, vocab, layers=1, max_batch=64, rope_style=0, weights="bf16", oracle=None):
+    """A model of full width with bf16 projections (or int8 ones) and a bf16 head, random norm weights; its oracle beside it."""
+    from paged_infer_b200 import api
+    from paged_infer_b200.loader import HostWeights, LlamaConfig, f32_to_bf16_bits
+    cfg = LlamaConfig(hidden, layers, heads, kv_heads, inter, vocab, 1e-5, 10000.0)
+    cfg.rope_style = rope_style
+    kv = kv_heads * (hidden // heads)
+    shapes = {"wq": (hidden, hidden), "wk": (kv, hidden), "wv": (kv, hidden), "wo": (hidden, hidden), "w1": (inter, hidden),
+              "w2": (hidden, inter), "w3": (inter, hidden)}
+
+    def matrix(shape, i):
+        w = normal_f32(shape, seed * 1000 + i, 0.02)
+        return f32_to_bf16_bits(w) if weights == "bf16" else oracle.quantize_rows_i8(w, *shape)
+
+    projs = [{k: matrix(s, l * 10 + j) for j, (k, s) in enumerate(shapes.items())} for l in range(layers)]
+    norms = [(1.0 + normal_f32((hidden,), seed * 1000 + 900 + i, 0.2)).astype(np.float32) for i in range(2 * layers + 1)]
+    head = f32_to_bf16_bits(normal_f32((vocab, hidden), seed * 1000 + 999, 0.02))
+    hw = HostWeights(f32_to_bf16_bits(normal_f32((vocab, hidden), seed * 1000 + 998, 0.5)), norms[0], norms[1:layers + 1], norms[layers + 1:], projs, None)
+    om = oracle and oracle.Model(cfg.as_dict(), hw.token_embeddings, hw.final_norm, hw.attention_norm, hw.ffn_norm, projs, head)
+    return cfg, om, api.LlamaWeights(ctx, cfg, hw, max_batch=max_batch, lm_head=head)
+
+
+def test_model_chunk_larger_than_a_portion(ctx):
+    """A chunk of 1300 rows of a bf16 model: the first layer's [q;k;v] goes through the scratch in two portions, with the rotary
+    embedding and the KV write of each; the CUDA-core kernels on the same inputs."""
+    from paged_infer_b200 import api
+    cfg, _, gm = bf16_llama(ctx, 51, 1024, 16, 4, 2816, 2048, layers=2, max_batch=1300)
+    n, block, nblocks = 1300, 16, 90
+    rng = np.random.default_rng(2)
+    prompt, table = rng.integers(0, cfg.vocab_size, n).astype(np.uint32), [int(b) for b in rng.permutation(nblocks)[:n // block + 1]]
+    got = []
+    for tensor in (1, 0):
+        ctx.set_option(1, tensor)                       # PI_OPT_TENSOR_GEMM
+        gkv = api.KvCache(ctx, gm.kv_layout(nblocks, block))
+        gkv.upload(np.zeros(gm.kv_layout(nblocks, block).total_floats(), np.float32))
+        got.append((gm.prefill_batched(prompt, 0, table, gkv, n), gkv.download()))
+    ctx.set_option(1, 1)
+    for a, b in zip(*got):                              # five projections in a row, each a few 2^-24 off on either side
+        assert np.abs(a - b).max() < 2e-5 * np.sqrt((b.astype(np.float64) ** 2).mean())
