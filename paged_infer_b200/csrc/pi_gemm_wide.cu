@@ -22,8 +22,8 @@
 // threads ask for the next stage before they work on this one.  24000 x 5600, alone: 85 us for 64 rows, 77 us for 5 (41 us
 // is the matrix out of HBM); the CUDA-core kernel takes 755 and 104.
 //
-// Warps 0-7: epilogue; 8: TMA; 9: tensor memory and MMA issue.  Waits are bounded as in pi_gemm_tc.cu; one that runs out
-// sets the context's error word, and tickets are taken all the same, so that the counters are zero again behind every
+// Warps 0-7: epilogue; 8: TMA; 9: tensor memory and MMA issue.  Waits are bounded; one that runs out sets the context's error
+// word and ends the CTA's other waits, and tickets are taken all the same, so that the counters are zero again behind every
 // launch.
 #include <algorithm>
 
@@ -36,6 +36,7 @@ namespace {
 using namespace pi_tc;
 using pi_wide::Cut;
 using pi_wide::cut_at;
+using pi_wide::kGivenUp;
 
 constexpr int kWR = pi_wide::kRows, kWC = pi_wide::kCols, kWK = pi_wide::kBlock;
 constexpr int kStages = 4, kDrain = 8, kWideThreads = (kDrain + 2) * 32;
@@ -63,7 +64,7 @@ gemm_wide_kernel(const GemmParams p, const Cut cut, float* __restrict__ parked, 
   float* tile_out = reinterpret_cast<float*>(smem + (size_t)kStages * kStageBytes);   // [64 activation rows][128 weight rows]
   __shared__ __align__(8) unsigned long long bars[2 * kStages + 4];
   __shared__ uint32_t s_tmem;
-  __shared__ volatile int s_abort, s_dep_ok;
+  __shared__ volatile int s_weight;
   __shared__ EpiPlace s_place[kWC];
   __shared__ int s_n, s_slots[pi_wide::kMaxHolders];
 
@@ -82,8 +83,7 @@ gemm_wide_kernel(const GemmParams p, const Cut cut, float* __restrict__ parked, 
       mbar_init(d_full + 8 * b, 1);
       mbar_init(d_empty + 8 * b, kDrain);
     }
-    s_abort = 0;
-    s_dep_ok = 0;
+    s_weight = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -97,9 +97,12 @@ gemm_wide_kernel(const GemmParams p, const Cut cut, float* __restrict__ parked, 
   pi_grid_launch_dependents();   // only now that this CTA holds its tensor memory
   const uint32_t tmem = s_tmem, smem_base = smem_u32(smem);
 
+  auto wait = [&](uint32_t bar, uint32_t parity) {
+    return pi_wide::wait_for([&] { return mbar_test(bar, parity); }, &s_weight);
+  };
   auto give_up = [&](int code) {
-    if (!s_abort && p.err_flag) atomicExch(p.err_flag, code);
-    s_abort = 1;
+    if (s_weight != kGivenUp && p.err_flag) atomicExch(p.err_flag, code);
+    s_weight = kGivenUp;   // the copying thread's 1 is not ahead of us: only waits that counted can run out
   };
 
   if (warp == kTma) {
@@ -121,12 +124,12 @@ gemm_wide_kernel(const GemmParams p, const Cut cut, float* __restrict__ parked, 
       const int n = pos1 - pos0, ahead = min(n, kStages);
       for (int it = 0; it < ahead; ++it) load_w(it, (pos0 + it) / nkb, (pos0 + it) % nkb);   // weights never depend on the preceding kernel
       pi_grid_dependency_wait();
-      s_dep_ok = 1;
+      s_weight = 1;
       int it = 0;
       bool free_next = false;   // the next stage is known to be free
       for (; it < n; ++it) {
         if (it >= ahead) {
-          if ((!free_next && !mbar_wait_dep(empty + 8 * (it % kStages), ((it / kStages) & 1) ^ 1, &s_dep_ok)) || s_abort) {
+          if ((!free_next && !wait(empty + 8 * (it % kStages), ((it / kStages) & 1) ^ 1)) || s_weight == kGivenUp) {
             give_up(32);
             break;
           }
@@ -139,7 +142,7 @@ gemm_wide_kernel(const GemmParams p, const Cut cut, float* __restrict__ parked, 
           ++tile;
         }
       }
-      if (s_abort)   // no copy of this CTA may still be in flight when it leaves
+      if (s_weight == kGivenUp)   // no copy of this CTA may still be in flight when it leaves
         for (int i = max(0, it - kStages); i < it; ++i) mbar_wait(full + 8 * (i % kStages), (i / kStages) & 1);
     }
   } else if (warp == kMma) {
@@ -150,9 +153,10 @@ gemm_wide_kernel(const GemmParams p, const Cut cut, float* __restrict__ parked, 
       bool full_next = false, d_next = true;   // the next stage, the next accumulator are known to be ready
       for (int it = 0; it < n; ++it) {
         const int s = it % kStages, buf = it & 1;
-        if ((!d_next && !mbar_wait_dep(d_empty + 8 * buf, ((it >> 1) & 1) ^ 1, &s_dep_ok)) ||
-            (!full_next && !mbar_wait_dep(full + 8 * s, (it / kStages) & 1, &s_dep_ok)) || s_abort) {
+        if ((!d_next && !wait(d_empty + 8 * buf, ((it >> 1) & 1) ^ 1)) ||
+            (!full_next && !wait(full + 8 * s, (it / kStages) & 1)) || s_weight == kGivenUp) {
           give_up(33);
+          if (it > 0) mbar_wait(d_full + 8 * (buf ^ 1), ((it - 1) >> 1) & 1);   // products under way still use the tensor memory
           break;
         }
         full_next = mbar_test(full + 8 * ((it + 1) % kStages), ((it + 1) / kStages) & 1);
@@ -183,7 +187,7 @@ gemm_wide_kernel(const GemmParams p, const Cut cut, float* __restrict__ parked, 
         const int buf = it & 1;
         int got = 0;
         if (lane == 0) {
-          got = (mbar_wait_dep(d_full + 8 * buf, (it >> 1) & 1, &s_dep_ok) && !s_abort) ? 1 : 0;
+          got = (wait(d_full + 8 * buf, (it >> 1) & 1) && s_weight != kGivenUp) ? 1 : 0;
           if (!got) give_up(35);
         }
         got = __shfl_sync(0xffffffffu, got, 0);

@@ -17,6 +17,20 @@ constexpr int kMinPart = 4;      // a share's end closer than this many blocks t
 constexpr int kMaxShare = 8;     // CTAs per tile at most, on average
 constexpr int kMaxHolders = 16;  // CTAs that can hold parts of one tile
 
+// A bounded wait.  `*weight` is what a poll counts: 0 while the kernel ahead still runs (those polls are not this launch's), then
+// 1, and the whole limit once a wait of the CTA has run out, so that from then on a wait ends with its first poll that fails:
+// however many K blocks are left, what a CTA still has to do are its tickets.  (With a comparison of its own for that the loop
+// answers later: 2 % of a launch.)
+constexpr int kPollLimit = 1 << 21, kGivenUp = kPollLimit;
+template <class Done>
+__device__ inline bool wait_for(Done done, const volatile int* weight) {
+  for (int spin = 0; spin < kPollLimit;) {
+    if (done()) return true;
+    spin += *weight;
+  }
+  return false;
+}
+
 // Tiles in order (row tile, column tile), K blocks innermost, all in one line; CTA i takes [cut_at(i), cut_at(i + 1)).
 struct Cut {
   int tiles, mtiles, nkb, ctas;

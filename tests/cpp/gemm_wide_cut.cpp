@@ -34,8 +34,29 @@ static void portions() {
   std::printf("ok portions\n");
 }
 
+// A CTA of many blocks whose products stop coming: one wait runs out, every later one costs a single poll.
+static void giving_up() {
+  volatile int weight = 1;
+  const int limit = kPollLimit, blocks = 2000, reached = 37;
+  int done = 0, polls = 0;
+  for (int it = 0; it < blocks; ++it) {   // the epilogue walks on to its tickets
+    if (wait_for([&] { ++polls; return it < reached; }, &weight) && weight != kGivenUp)
+      ++done;
+    else
+      weight = kGivenUp;
+  }
+  CHECK(done == reached && polls == reached + limit + (blocks - reached - 1));
+  weight = polls = 0;                     // polls ahead of the dependency do not count
+  CHECK(wait_for([&] { weight = ++polls > 3 * limit; return polls == 3 * limit + 7; }, &weight));
+  weight = 1;
+  polls = 0;                              // another warp gives up meanwhile
+  CHECK(!wait_for([&] { weight = ++polls == 9 ? kGivenUp : 1; return false; }, &weight) && polls == 9);
+  std::printf("ok giving up\n");
+}
+
 int main() {
   portions();
+  giving_up();
   if (!failures) std::printf("all ok\n");
   return failures != 0;
 }
