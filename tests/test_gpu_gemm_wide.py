@@ -203,3 +203,26 @@ def test_model_chunk_larger_than_a_portion(ctx):
     ctx.set_option(1, 1)
     for a, b in zip(*got):                              # five projections in a row, each a few 2^-24 off on either side
         assert np.abs(a - b).max() < 2e-5 * np.sqrt((b.astype(np.float64) ** 2).mean())
+
+
+def test_infinite_weights(ctx):
+    """Weights that are infinite or NaN give what 64 bits and the CUDA-core kernel give, and touch their own columns only."""
+    from paged_infer_b200 import api
+    bits, w = bf16_matrix(4096, 2048, 11)
+    x = normal_f32((70, 2048), 12, 1.0)
+    x[9, 100], x[10, 100] = 0.0, np.inf
+    x[:, 2047] = np.float32(1.5)                     # exactly one bf16: the other planes are zero
+    for row, col, value in [(3, 100, np.inf), (130, 7, -np.inf), (131, 7, np.nan), (4000, 2047, np.inf)]:
+        w[row, col] = value
+        bits[row, col] = {np.inf: 0x7f80, -np.inf: 0xff80}.get(value, 0x7fc0)
+    w[4000, 3], bits[4000, 3] = -np.inf, 0xff80      # two signs in one row: NaN where both act in one direction
+    with np.errstate(invalid="ignore"):
+        want = x.astype(np.float64) @ w.astype(np.float64).T
+    for tensor in (1, 0):                            # PI_OPT_TENSOR_GEMM
+        ctx.set_option(1, tensor)
+        got = api.Projection.f32(ctx, bits).apply_batched(x)
+        ctx.set_option(1, 1)
+        finite = np.isfinite(want)
+        assert np.array_equal(got[~finite], want[~finite].astype(np.float32), equal_nan=True)
+        norm = np.sqrt((np.where(finite, want, 0) ** 2).mean(axis=1, keepdims=True))
+        assert (np.abs(got[finite] - want[finite]) / np.maximum(np.abs(want), norm)[finite]).max() < 2e-6
