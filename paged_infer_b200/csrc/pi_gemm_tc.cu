@@ -714,13 +714,9 @@ bool pi_gemm_tc_supported(const pi_ctx* ctx, const pi_linear* lin, const pi_line
     if ((uintptr_t)lin->w % 32 != 0) return false;
   } else if (lin->kind == PI_BF16) {
     if (!wide_fits(lin)) return false;
-    // The CUDA-core kernel takes about 4 us and 0.37 us per million weights and pass over four rows, the split and the
-    // tensor-core GEMM 13 us and 0.5 us per million weights, whatever the batch: the lines cross where a million weights
-    // times (3 passes - 4) reach 70.  Both sides, us: 2048 x 2048, 32 rows (84) 17.9 and 16.2, 16 rows (34) 10.6 and 14.7;
-    // 11264 x 2048, 8 rows (46) 21.7 and 23.9, 16 rows (185) 39.9 and 24.6; 24000 x 5600, 5 rows (269) 104 and 77.
-    const double weights = (double)lin->rows * (double)lin->cols, passes = (a.M + 3) / 4;
-    if (weights * (3 * passes - 4) < 70e6) return false;
-    if (weights * ((a.M + 63) / 64) >= 8e12) return false;   // K blocks of a launch are counted in 32 bits
+    if (!pi_wide::worth(lin->rows, lin->cols, a.M, ctx->sm_count, ctx->smem_optin - 2048)) return false;
+    // K blocks of a launch are counted in 32 bits
+    if ((double)lin->rows * (double)lin->cols * ((a.M + 63) / 64) >= 8e12) return false;
     if (!ctx->gemm_parked.ptr || ctx->wide_planes.bytes < pi_wide::planes_bytes(pi_wide::portion_rows(a.M, lin->cols), lin->cols)) return false;
   } else {
     return false;

@@ -75,6 +75,28 @@ __host__ __device__ inline int holders(const Cut& c, int cta, int tile, int* slo
   return n;
 }
 
+// Which kernel a call takes, of two that both could: true for this one.  Times in us, device, matrices out of HBM, both sides
+// measured over 32..28672 rows, 1024..28672 columns and batches of 5 to 512, activations split by a launch of their own.
+// The CUDA-core kernel takes 4 and 0.37 per million weights and pass over four activation rows (0.44 where one CTA of it fills
+// an SM); rows too long for four in shared memory make passes over two (0.30) or one (0.18).
+// On a full grid this one with the split takes 13 and 0.5 per million weights for up to 64 activation rows: the lines cross where
+// a million weights times (3 passes - 4) reach 70.  2048 x 2048, 32 rows (84) 18.5 and 16.2, 16 rows (34) 10.9 and 15.0;
+// 11264 x 2048, 8 rows (46) 22.8 and 24.3, 16 rows (185) 41.5 and 25.0; 24000 x 5600, 5 rows (269) 104 and 75.
+// Few rows of many columns leave it few CTAs with long shares: 8, a microsecond per 1600 columns for the split (twice that beyond
+// 16384, where a row leaves the registers) and 0.55 per K block of a share.  32 x 28672, 256 rows 54 and 96; 128 x 28672,
+// 32 rows 39 and 68; 2048 x 28672, 5 rows 82 and 100.  Near a draw (1.2) the first line decides.
+inline bool worth(size_t rows, size_t cols, int M, int sms, size_t smem) {
+  int group = M >= 4 ? 4 : M >= 2 ? 2 : 1;
+  while (group > 1 && group * cols * sizeof(float) > smem) group >>= 1;
+  if (group * cols * sizeof(float) > smem) return true;   // the CUDA-core kernel has no room for a row
+  const double mega = 1e-6 * (double)rows * (double)cols, fours = (M - 1) / 4 + 1, passes = (M - 1) / group + 1;
+  if (mega * (3 * fours - 4) < 70) return false;
+  const double cores = 4 + mega * passes * (group == 1 ? 0.18 : group == 2 ? 0.30 : cols > 7000 ? 0.44 : 0.37);
+  const Cut c = make_cut((int)rows, M, (int)cols, sms);
+  const double tensor = 8 + (double)cols / (cols > 16384 ? 800 : 1600) + 0.55 * c.tiles * c.nkb / c.ctas;
+  return 1.2 * cores > tensor;
+}
+
 // Scratch for the activations of a launch: three 16-bit planes and a factor per row.
 inline size_t planes_bytes(size_t rows, size_t cols) { return 3 * rows * cols * 2 + rows * sizeof(float) + 256; }
 

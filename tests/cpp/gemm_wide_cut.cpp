@@ -54,7 +54,29 @@ static void giving_up() {
   std::printf("ok giving up\n");
 }
 
+// The dispatch line against both sides as measured (us): the chosen side is never more than a quarter slower than the other.
+static void dispatch() {
+  const struct { int rows, cols, M; double cores, tensor; } seen[] = {
+      {32, 1024, 512, 4.4, 16.3},       {32, 16384, 64, 15.8, 36.7},     {32, 16384, 256, 31.9, 40.3},     {32, 28672, 64, 24.8, 70.3},
+      {32, 28672, 128, 39.0, 71.2},     {32, 28672, 256, 53.8, 96.0},    {64, 5632, 512, 24.1, 25.2},      {128, 2048, 64, 9.7, 16.8},
+      {128, 8192, 512, 67.5, 30.0},     {128, 28672, 5, 14.3, 65.3},     {128, 28672, 32, 39.0, 68.0},     {128, 28672, 64, 81.2, 73.4},
+      {128, 28672, 512, 336.5, 116.0},  {256, 2048, 512, 33.3, 19.4},    {256, 8192, 128, 38.3, 27.2},     {512, 1024, 64, 6.9, 15.3},
+      {512, 4096, 64, 18.2, 21.9},      {512, 4096, 512, 111.4, 30.0},   {1024, 2048, 32, 10.8, 15.9},     {1024, 2048, 128, 32.5, 18.3},
+      {1024, 8192, 5, 20.6, 23.4},      {1024, 8192, 64, 67.5, 27.9},    {2048, 2048, 16, 10.9, 15.0},     {2048, 2048, 32, 18.5, 16.2},
+      {2048, 5632, 8, 16.2, 20.8},      {2048, 5632, 24, 33.4, 22.4},    {2560, 2048, 16, 14.1, 15.4},     {2560, 2048, 24, 18.5, 16.0},
+      {4096, 4096, 5, 18.7, 23.8},      {4096, 4096, 16, 32.1, 26.7},    {11264, 2048, 8, 22.8, 24.3},     {11264, 2048, 12, 33.7, 24.6},
+      {2048, 28672, 5, 82.3, 100.4},    {2048, 28672, 16, 175.3, 101.3}, {24000, 5600, 5, 104.4, 75.1},    {28672, 4096, 8, 91.1, 67.3}};
+  for (const auto& s : seen) {
+    const bool tensor = worth(s.rows, s.cols, s.M, 148, 232448 - 2048);
+    const double took = tensor ? s.tensor : s.cores, other = tensor ? s.cores : s.tensor;
+    if (took > 1.25 * other) std::printf("FAILED %d x %d, %d rows: %.1f taken, %.1f not\n", s.rows, s.cols, s.M, took, other), ++failures;
+  }
+  CHECK(worth(40, 65536, 5, 148, 232448 - 2048));   // rows that the CUDA-core kernel refuses
+  std::printf("ok dispatch\n");
+}
+
 int main() {
+  dispatch();
   portions();
   giving_up();
   if (!failures) std::printf("all ok\n");
