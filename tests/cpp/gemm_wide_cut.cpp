@@ -1,6 +1,8 @@
-// The scratch of the GEMM for bf16 weights (csrc/pi_gemm_wide.cuh), without a GPU.  Prints "ok <name>" per group; exit code 0 only
+// The cut and the scratch of the GEMM for bf16 weights (csrc/pi_gemm_wide.cuh), without a GPU.  Prints "ok <name>" per group; exit code 0 only
 // if every check held.
 #include <cstdio>
+#include <random>
+#include <vector>
 
 #include "../../paged_infer_b200/csrc/pi_gemm_wide.cuh"
 
@@ -14,6 +16,51 @@ static int failures = 0;
       ++failures;                                                   \
     }                                                               \
   } while (0)
+
+// Every K block of every tile belongs to one CTA; the holders of a tile agree on slots, order and counter; no two tiles share a
+// parking slot or a counter.
+static void cut() {
+  std::mt19937 rng(1);
+  auto between = [&](int lo, int hi) { return (int)(lo + rng() % (unsigned)(hi - lo + 1)); };
+  for (int round = 0; round < 1500; ++round) {
+    const int sms = round % 3 ? 148 : between(1, 160), big = round % 5 == 0;
+    const Cut c = make_cut(between(32, big ? 40000 : 3000), between(5, big ? 1300 : 200), 8 * between(1, round % 7 == 0 ? 16384 : 700), sms);
+    CHECK(c.ctas >= 1 && c.ctas <= sms && cut_at(c, 0) == 0 && cut_at(c, c.ctas) == c.tiles * c.nkb);
+    std::vector<int> counter(c.ctas, -1), slot(2 * c.ctas, -1);
+    std::vector<std::vector<int>> seen(c.tiles);
+    for (int i = 0; i < c.ctas; ++i) {
+      const int pos0 = cut_at(c, i), pos1 = cut_at(c, i + 1);
+      CHECK(pos0 <= pos1);
+      for (int pos = pos0; pos < pos1;) {
+        const int tile = pos / c.nkb, first = tile * c.nkb, end = first + c.nkb < pos1 ? first + c.nkb : pos1;
+        if (pos != first || end != first + c.nkb) {   // a part
+          const int mine = i * 2 + (pos0 >= first ? 0 : 1);
+          CHECK(slot[mine] == -1);
+          slot[mine] = tile;
+          int slots[kMaxHolders], j0 = -1;
+          const int n = holders(c, i, tile, slots, &j0);
+          CHECK(n >= 2 && n <= kMaxHolders && j0 >= 0 && j0 < c.ctas);
+          CHECK(counter[j0] == -1 || counter[j0] == tile);
+          counter[j0] = tile;
+          std::vector<int> all(slots, slots + n);
+          bool holds = false;
+          for (int k = 0; k < n; ++k) {
+            holds = holds || all[k] == mine;
+            CHECK(k == 0 || all[k] / 2 > all[k - 1] / 2);
+          }
+          CHECK(holds && (seen[tile].empty() || seen[tile] == all));
+          seen[tile] = all;
+        } else {
+          CHECK(seen[tile].empty());
+        }
+        pos = end;
+      }
+    }
+    for (int t = 0; t < c.tiles; ++t)
+      for (int s : seen[t]) CHECK(slot[s] == t);   // whoever is last reads what that CTA parked for this tile
+  }
+  std::printf("ok cut\n");
+}
 
 // Every call passes through the scratch that was laid out for its matrix, whatever its batch: equal portions of whole tiles.
 static void portions() {
@@ -76,6 +123,7 @@ static void dispatch() {
 }
 
 int main() {
+  cut();
   dispatch();
   portions();
   giving_up();

@@ -22,6 +22,6 @@ def lines(tmp_path_factory):
     return r.stdout.split("\n")
 
 
-@pytest.mark.parametrize("name", ["portions", "giving up", "dispatch"])
+@pytest.mark.parametrize("name", ["cut", "portions", "giving up", "dispatch"])
 def test_plan(lines, name):
     assert f"ok {name}" in lines and not any(l.startswith("FAILED") for l in lines)

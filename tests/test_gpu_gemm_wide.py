@@ -1,5 +1,7 @@
 """The tcgen05 GEMM for bf16 weights and f32 activations (projections of more rows than the CUDA-core kernel is for): against
-64 bits at the edges of its tiles (128 weight rows, 64 activation rows, 64 columns) and of its cut over the SMs.
+64 bits at the edges of its tiles (128 weight rows, 64 activation rows, 64 columns) and of its cut over the SMs, and, through
+models of full width against the oracle, every epilogue that it has (residual add, SwiGLU, rotary embedding and cache write,
+planes and sums of squares for the next projection).
 
 Tolerance, per activation row: the activations enter as three bf16 planes whose sum is the f32 value, products are exact, and
 single K blocks are summed in f32 by the tensor pipe, so that the error of a result is a few 2^-24 of the 2-norm of its row;
@@ -43,6 +45,11 @@ def test_bf16_weights(ctx, rows, cols, M):
     assert np.array_equal(got, p.apply_batched(x))   # a tile's parts are summed in one order
     norm = np.sqrt((want ** 2).mean(axis=1, keepdims=True))
     assert float((np.abs(got - want) / np.maximum(np.abs(want), norm)).max()) < 2e-6
+    # As a whole, where sums over blocks that are lost show: a running sum on the tensor pipe is cut by 1.5e-8 of itself every 16
+    # columns (2e-6 over 2048), those of single blocks 1.3e-7 at most; f32 sums of the blocks add 2^-25 a block at random.
+    rest = slice(1, M - 1)
+    bound = 2 * np.hypot(1.3e-7, 2.0 ** -25 * np.sqrt(cols / 64) / 2)
+    assert np.linalg.norm((got - want)[rest]) < bound * np.linalg.norm(want[rest])
 
 
 def test_infinities_and_nan_stay_in_their_rows(ctx):
@@ -226,3 +233,70 @@ def test_infinite_weights(ctx):
         assert np.array_equal(got[~finite], want[~finite].astype(np.float32), equal_nan=True)
         norm = np.sqrt((np.where(finite, want, 0) ** 2).mean(axis=1, keepdims=True))
         assert (np.abs(got[finite] - want[finite]) / np.maximum(np.abs(want), norm)[finite]).max() < 2e-6
+
+
+# hidden 2048: heads of 64, whole tiles, rotary embedding in the epilogue; hidden 2000: heads of 80 (rotary embedding behind it),
+# no matrix a multiple of the tile; int8 layers under a bf16 head
+MODELS = [dict(hidden=2048, heads=32, kv_heads=4, inter=5632, vocab=4096), dict(hidden=2048, heads=16, kv_heads=4, inter=2824, vocab=4100, rope_style=1),
+          dict(hidden=2000, heads=25, kv_heads=5, inter=2824, vocab=4100, rope_style=1), dict(hidden=2048, heads=32, kv_heads=4, inter=2816, vocab=8200, weights="int8")]
+
+
+@pytest.fixture(scope="module", params=range(len(MODELS)))
+def bf16_model(request, ctx, oracle):
+    return MODELS[request.param], bf16_llama(ctx, 61 + request.param, layers=2, max_batch=130, oracle=oracle, **MODELS[request.param])
+
+
+def close_to_oracle(got, want, depth=8):
+    """Logits (or cache contents) behind `depth` projections in a row: the 2-norm of each one's error is 2e-7 of its result on either
+    side and the norms, gates and attention between them pass it on about as it is; values within six of their deviations."""
+    scale = np.sqrt((want.astype(np.float64) ** 2).mean())
+    return np.abs(got - want).max() < 2 * depth * 2e-7 * 6 * scale
+
+
+@pytest.mark.parametrize("chunk", [100, 130])
+def test_model_prefill(ctx, bf16_model, chunk):
+    """A prompt of 230 in chunks that are no multiple of a tile of 64 rows; logits and the cache."""
+    from paged_infer_b200 import api
+    kind, (cfg, om, gm) = bf16_model
+    n, block, nblocks = 230, 16, 18
+    rng = np.random.default_rng(4)
+    prompt, table = rng.integers(0, cfg.vocab_size, n).astype(np.uint32), [int(b) for b in rng.permutation(nblocks)[:n // block + 1]]
+    layout = gm.kv_layout(nblocks, block)
+    okv, gkv = np.zeros(layout.total_floats(), np.float32), api.KvCache(ctx, layout)
+    gkv.upload(okv)
+    want = om.prefill_batched(prompt, 0, table, okv, block, 32)
+    ctx.profile_begin()
+    got = gm.prefill_batched(prompt, 0, table, gkv, chunk)
+    assert ctx.profile_end()["gemm_tc"][1] == 8 * -(-n // chunk)     # every projection but the head of the last row
+    assert close_to_oracle(got, want)
+    assert close_to_oracle(gkv.download()[okv != 0], okv[okv != 0])
+
+
+@pytest.mark.parametrize("batch", [8, 12, 24, 64])
+def test_model_decode(ctx, oracle, bf16_model, batch):
+    """Batches on both sides of the dispatch line and across it (some projections of a layer on each kernel): a step with logits, then
+    greedy steps, the later ones out of a captured graph."""
+    from paged_infer_b200 import api
+    kind, (cfg, om, gm) = bf16_model
+    block, nblocks, steps = 16, 3 * batch, 6
+    rng = np.random.default_rng(5)
+    layout = gm.kv_layout(nblocks, block)
+    okv = (rng.standard_normal(layout.total_floats()) * 0.5).astype(np.float32)
+    before, gkv = okv.copy(), api.KvCache(ctx, layout)
+    gkv.upload(okv)
+    tables = [[int(x) for x in row] for row in rng.permutation(nblocks).reshape(batch, 3)]
+    tokens, pos = [int(t) for t in rng.integers(0, cfg.vocab_size, batch)], [int(p) for p in rng.integers(0, 40, batch)]
+    want = om.decode_batch(tokens, pos, tables, okv, block)
+    ctx.profile_begin()
+    got = gm.decode_batch_into(tokens, pos, tables, gkv, want_logits=True)
+    tensor = ctx.profile_end()["gemm_tc"][1]
+    assert tensor == 9 if batch == 64 or (kind.get("weights") == "int8" and batch >= 12) else tensor < 9
+    assert close_to_oracle(got, want)
+    ids = gm.decode_multi(tokens, pos, tables, gkv, steps)
+    for i in range(steps):
+        want = om.decode_batch(tokens, [p + i for p in pos], tables, okv, block)
+        tokens = [oracle.argmax(r) for r in want]
+        assert ids[i].tolist() == tokens
+    wrote, after = okv != before, gkv.download()
+    assert np.array_equal(after[~wrote], okv[~wrote])
+    assert close_to_oracle(after[wrote], okv[wrote])    # against the size of what was written, not of the rest of the cache
