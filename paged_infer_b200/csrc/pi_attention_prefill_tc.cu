@@ -129,8 +129,9 @@ __device__ __forceinline__ void t_ld64(uint32_t base, float* v) {
 #pragma unroll
   for (int i = 0; i < 64; ++i) v[i] = __uint_as_float(r[i]);
 }
-// The three planes of a pair of values, packed (x in the low half): same roundings as pi_split3, two values per
-// conversion instruction.
+// The three planes of a pair of values, packed (x in the low half), two values per conversion instruction: the roundings of
+// pi_split3 below the values that round beyond the largest bf16 (3.3962e38).  From there on, infinities included, the first
+// plane is infinite here and the others are infinite or NaN.
 __device__ __forceinline__ void split3_pair(float x, float y, uint32_t& w0, uint32_t& w1, uint32_t& w2) {
   __nv_bfloat162 a = __floats2bfloat162_rn(x, y);
   w0 = *reinterpret_cast<uint32_t*>(&a);

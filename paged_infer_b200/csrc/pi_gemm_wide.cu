@@ -19,8 +19,8 @@
 // (K 5600: 1.7e-7 and 1.8e-7).
 //
 // What bounds it: hand-overs.  A wait on an mbarrier takes about 190 cycles even when the phase is complete, so the issuing
-// threads ask for the next stage before they work on this one.  24000 x 5600, alone: 85 us for 64 rows, 77 us for 5 (41 us
-// is the matrix out of HBM); the CUDA-core kernel takes 755 and 104.
+// threads ask for the next stage before they work on this one.  24000 x 5600, alone, with the split: 83 us for 64 rows, 76 us for 5
+// (42 us is the matrix out of HBM); the CUDA-core kernel takes 755 and 104.
 //
 // Warps 0-7: epilogue; 8: TMA; 9: tensor memory and MMA issue.  Waits are bounded; one that runs out sets the context's error
 // word and ends the CTA's other waits, and tickets are taken all the same, so that the counters are zero again behind every
